@@ -61,13 +61,16 @@ __device__ __forceinline__ double fused_value(const FusedArgs &a, int32_t g, flo
 // Rows of W and G are read from copies padded with zeros to 4 LPR floats
 // (LPR = 8, 16 or 32 lanes, k <= 32, 64 or 128): LPR lanes take a row as one
 // 16-byte load each, so a row is whole 128-byte lines and a warp works on
-// 32 / LPR entries at a time, four columns per lane.
-__global__ void k_pad_rows(const float *__restrict__ in, int64_t rows, int k, int kp, float *__restrict__ out) {
+// 32 / LPR entries at a time, four columns per lane.  The copy has a row 0
+// even when there are no rows (d = 0): slots without an entry, and entries
+// whose gene id is outside [0, d), load that row and drop what they load.
+__global__ void k_pad_rows(const float *__restrict__ in, int64_t rows, int64_t rows_out, int k, int kp,
+                           float *__restrict__ out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * kp) return;
+    if (i >= rows_out * kp) return;
     const int64_t r = i / kp;
     const int j = (int)(i - r * kp);
-    out[i] = j < k ? in[r * k + j] : 0.0f;
+    out[i] = r < rows && j < k ? in[r * k + j] : 0.0f;
 }
 
 // One entry of the W gradient: s_e and its cell.
@@ -500,9 +503,9 @@ struct FusedWork {
 int padded_columns(int64_t k) { return k <= 32 ? 32 : k <= 64 ? 64 : 128; }
 
 int pad_rows(const float *in, int64_t rows, int64_t k, int kp, DevBuf &buf, cudaStream_t st) {
-    CREST_TRY(buf.ensure(sizeof(float) * (size_t)std::max<int64_t>(rows * kp, 1)));
-    if (rows > 0)
-        k_pad_rows<<<(unsigned)ceil_div(rows * kp, 256), 256, 0, st>>>(in, rows, (int)k, kp, buf.as<float>());
+    const int64_t rows_out = std::max<int64_t>(rows, 1);
+    CREST_TRY(buf.ensure(sizeof(float) * (size_t)(rows_out * kp)));
+    k_pad_rows<<<(unsigned)ceil_div(rows_out * kp, 256), 256, 0, st>>>(in, rows, rows_out, (int)k, kp, buf.as<float>());
     CREST_CUDA_TRY(cudaGetLastError());
     return CREST_OK;
 }

@@ -118,3 +118,35 @@ def test_few_cells_spread_over_blocks(n, d, k, per):
     assert rel(gx, rx) <= 1e-4
     assert rel(gsf, rsf) <= 1e-4
     assert rel(gW, rW) <= 1e-4
+
+
+@pytest.mark.parametrize("k", [1, 50, 128])
+@pytest.mark.parametrize("n", [40, 5000])
+def test_no_genes(n, k):
+    """d = 0 through the C interface: entries are rejected (no gene id is in
+    range) without a row of W being read - the padded copy has a zero row 0 for
+    them - and an empty matrix has zero scores and gradients."""
+    dev = torch.device("cuda")
+    per = 37
+    f32 = dict(dtype=torch.float32, device=dev)
+    W, mean = torch.full((4,), float("nan"), **f32), torch.zeros(1, dtype=torch.float64, device=dev)
+    sf, G = torch.ones(n, **f32), torch.ones((n, k), **f32)
+    indices, values = torch.zeros(n * per, dtype=torch.int32, device=dev), torch.ones(n * per, **f32)
+    for entries in (per, 0):
+        indptr = torch.arange(n + 1, device=dev) * entries
+        scores, gx, gsf = (torch.full(s, 7.0, **f32) for s in ((n, k), (n * per,), (n,)))
+        a = (indptr.data_ptr(), indices.data_ptr(), values.data_ptr(), n, 0, sf.data_ptr(), W.data_ptr(), k,
+             mean.data_ptr(), mean.data_ptr(), 10.0)
+        out = (G.data_ptr(), gx.data_ptr(), gsf.data_ptr(), W.data_ptr())
+        torch.cuda.synchronize()
+        if entries:
+            with pytest.raises(ValueError, match=r"gene ids in \[0, d\)"):
+                _lib.call("crest_fused_forward", *a, scores.data_ptr())
+            with pytest.raises(ValueError, match=r"gene ids in \[0, d\)"):
+                _lib.call("crest_fused_backward", *a, *out)
+        else:
+            _lib.call("crest_fused_forward", *a, scores.data_ptr())
+            _lib.call("crest_fused_backward", *a, *out)
+        assert torch.all(scores == 0) and torch.all(gsf == 0)
+        assert torch.all(gx[:n * entries] == 0)
+        assert torch.all(torch.isnan(W))  # an output of no rows, and an input of none
