@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kStatsThreads) k_gene_stats_csc(DevChunk c, co
                     const double scale = __ldg(cell_scale + cell[u]);
                     vf = transform_value(c, scale, x[u]);
                     ev = expm1((double)vf);
-                    use[u] = scale >= 0.0;
+                    use[u] = !(scale < 0.0);  // a cell whose factor is NaN is a kept one
                 } else {
                     use[u] = use[u] && ev != -2.0;
                 }

@@ -43,3 +43,20 @@ def test_gene_stats_around_the_table(n, n_genes, per_cell, target, log):
     oracle.gene_stats(idx, val, cm, gm, target, log, None, indptr, 0, ref)
     assert np.array_equal(got[:, 4], ref[:, 4])
     np.testing.assert_allclose(got[:, :4], ref[:, :4], rtol=1e-12, atol=1e-300)
+
+
+def test_gene_stats_of_a_cell_without_a_factor():
+    """An infinite total under an infinite target leaves a NaN factor: the
+    cell's entries count and make their genes' sums NaN, for counts inside and
+    outside the table alike."""
+    indptr = np.array([0, 4, 6], np.int64)
+    idx = np.array([0, 1, 2, 3, 1, 3], np.uint32)
+    val = np.array([np.inf, 1.0, 20.0, 2.5, 3.0, 40.0], np.float32)
+    cm, gm = np.arange(2, dtype=np.int64), np.arange(5, dtype=np.int32)
+    m = core.DeviceMatrix(indptr, idx, val, 5)
+    got, ref = np.zeros((5, 5)), np.zeros((5, 5))
+    _lib.call("crest_matrix_gene_stats", m.handle, _lib.ptr(cm), _lib.ptr(gm), np.inf, 1, 5, _lib.ptr(got))
+    m.close()
+    oracle.gene_stats(idx, val, cm, gm, np.inf, True, None, indptr, 0, ref)
+    assert np.array_equal(got[:, 4], ref[:, 4])
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
