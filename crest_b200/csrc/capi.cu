@@ -587,7 +587,7 @@ int crest_group_gene_sums(const crest_chunk *chunk, const uint32_t *group_of_row
     CREST_TRY(zeros<double>(x->out0, ne, st));
     if (sumsq) CREST_TRY(zeros<double>(x->out1, ne, st));
     if (nnz) CREST_TRY(zeros<uint32_t>(x->out2, ne, st));
-    CREST_TRY(launch_group_gene_sums(dc, nullptr, x->out5.as<uint32_t>(), n_vars, dclip, x->out0.as<double>(),
+    CREST_TRY(launch_group_gene_sums(dc, x->out5.as<uint32_t>(), n_vars, dclip, x->out0.as<double>(),
                                      sumsq ? x->out1.as<double>() : nullptr, nnz ? x->out2.as<uint32_t>() : nullptr,
                                      st));
     CREST_CUDA_TRY(cudaStreamSynchronize(st));  // a failed pass leaves the caller's sums as they are

@@ -7,26 +7,29 @@
 //   x = the lazily transformed value (normalize_total / log1p, f32),
 //   x = min(x, clip[group][gene]) when a clip table is given (seurat_v3),
 //   sum[group][gene] += x, sumsq += x * x, nnz += 1        (f64)
-// One warp per cell.  The transformed value of a count depends on the cell
-// only, so lane l evaluates that of l + 1 once per cell and an entry takes it
-// from there by a shuffle; other values are evaluated.  The cell's
-// normalisation factor comes from its kept-gene total when the caller has it
-// (resident matrices), else from a first read of the row.  Then, per entry,
-// two f64 atomics and one integer atomic into the (n_groups x n_vars) outputs,
-// which are small enough to stay in L2; these bound the pass (50,000 cells,
-// 73M entries: 1.27 ms with every entry evaluated and three f64 atomics,
-// 0.97 ms now with the totals at hand).  The reference sums each (group, gene) in entry order; here
-// the order of the atomics is not fixed, so results agree to rounding.
+// One warp per cell: the cell's normalisation factor from a first read of the
+// row (as every pass here; nothing is kept from one call for the next), then
+// the entries.  The transformed value of a count depends on the cell only, so
+// lane l evaluates that of l + 1 once per cell and an entry takes it from there
+// by a shuffle; other values are evaluated.  Per entry, two f64 atomics and one
+// integer atomic go to global memory: the (n_groups x n_vars) outputs stay in
+// L2, and these three updates of three arrays bound the pass, not the
+// evaluation they replace (50,000 cells, 70M entries, every cell in a group:
+// 1.22 ms, as with every entry evaluated and three f64 atomics; with a
+// twentieth of the cells in a group 125 us against 168).  The integer counts
+// also halve that part of the read-back.  The reference sums each (group, gene)
+// in entry order; here the order of the atomics is not fixed, so results agree
+// to rounding.
 #include "kernels.cuh"
 #include "prof.cuh"
 #include "rowwarp.cuh"
 
 namespace crest {
 
-__global__ void __launch_bounds__(256) k_group_gene_sums(DevChunk c, const double *__restrict__ total_of_span,
-                                                         const uint32_t *__restrict__ group_of_row, int64_t n_vars,
-                                                         const double *__restrict__ clip, double *__restrict__ sum,
-                                                         double *__restrict__ sumsq, uint32_t *__restrict__ nnz) {
+__global__ void __launch_bounds__(256) k_group_gene_sums(DevChunk c, const uint32_t *__restrict__ group_of_row,
+                                                         int64_t n_vars, const double *__restrict__ clip,
+                                                         double *__restrict__ sum, double *__restrict__ sumsq,
+                                                         uint32_t *__restrict__ nnz) {
     const int lane = lane_id();
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -36,13 +39,7 @@ __global__ void __launch_bounds__(256) k_group_gene_sums(DevChunk c, const doubl
         if (row < 0) continue;
         const uint32_t grp = __ldg(group_of_row + row);
         if (grp == 0xffffffffu) continue;
-        double scale = 1.0;
-        if (total_of_span && c.target_sum > 0.0) {
-            const double t = __ldg(total_of_span + i);
-            scale = t > 0.0 ? c.target_sum / t : 1.0;
-        } else {
-            scale = cell_scale(c, lo, hi);
-        }
+        const double scale = cell_scale(c, lo, hi);
         const float own = transform_value(c, scale, (float)(lane + 1));
         const int64_t base = (int64_t)grp * n_vars;
         for_entries<8>(c, lo, hi, [&](int32_t m, float xf) {
@@ -60,15 +57,15 @@ __global__ void __launch_bounds__(256) k_group_gene_sums(DevChunk c, const doubl
     }
 }
 
-int launch_group_gene_sums(const DevChunk &c, const double *total_of_span, const uint32_t *group_of_row, int64_t n_vars,
-                           const double *clip, double *sum, double *sumsq, uint32_t *nnz, cudaStream_t st) {
+int launch_group_gene_sums(const DevChunk &c, const uint32_t *group_of_row, int64_t n_vars, const double *clip,
+                           double *sum, double *sumsq, uint32_t *nnz, cudaStream_t st) {
     if (c.n_spans == 0) return CREST_OK;
     prof::Scope ps("group_gene_sums_csr", st);
     int64_t blocks = ceil_div(c.n_spans, 8);
     const int64_t cap = (int64_t)device_sms() * 16;
     if (blocks > cap) blocks = cap;
-    k_group_gene_sums<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(c, total_of_span, group_of_row, n_vars,
-                                                                              clip, sum, sumsq, nnz);
+    k_group_gene_sums<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(c, group_of_row, n_vars, clip, sum,
+                                                                              sumsq, nnz);
     CREST_CUDA_TRY(cudaGetLastError());
     return CREST_OK;
 }

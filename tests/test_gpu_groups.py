@@ -16,7 +16,7 @@ import pytest
 
 import crest_b200 as cb
 import oracle
-from crest_b200 import _native
+from crest_b200 import _lib, _native, core
 
 pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -141,3 +141,65 @@ def test_seurat_v3_matches_reference_golden(name, store):
         for col in ("means", "variances"):
             np.testing.assert_allclose(bf.var[col].to_numpy(), g[f"{tag}_{col}"], rtol=1e-12)
         np.testing.assert_allclose(bf.var["variances_norm"].to_numpy(), g[f"{tag}_variances_norm"], rtol=1e-9)
+
+
+def resident(m, cm, gm, target, log, grp, G, nv, cl=None):
+    out = [np.zeros((G, nv)) for _ in range(3)]
+    _lib.call("crest_matrix_group_gene_sums", m.handle, _lib.ptr(cm), _lib.ptr(gm), float(target), int(log), _lib.ptr(grp),
+              len(grp), G, nv, _lib.ptr(cl), *[_lib.ptr(a) for a in out])
+    return out
+
+
+@pytest.mark.parametrize("target,log", [(1e4, True), (0.0, True), (0.0, False)])
+@pytest.mark.parametrize("clip", [False, True])
+def test_resident_group_sums_around_the_lane_table(target, log, clip):
+    """Counts on both sides of the 32 that a warp tabulates, zeros and
+    fractions; a second gene map on the same matrix (other totals), then the
+    first again."""
+    rng = np.random.default_rng(31)
+    n, ng, per, G = 700, 400, 90, 6
+    idx = np.sort(rng.random((n, ng)).argpartition(per - 1, axis=1)[:, :per], axis=1).astype(np.uint32).ravel()
+    indptr = np.arange(n + 1, dtype=np.int64) * per
+    val = rng.choice(np.array([1, 2, 31, 32, 33, 0, 0.5, 31.5, 40000], np.float32), len(idx))
+    cm = np.arange(n, dtype=np.int64)
+    cm[::11] = -1
+    cm[cm >= 0] = np.arange((cm >= 0).sum())
+    nr = int(cm.max()) + 1
+    grp = rng.integers(0, G, nr).astype(np.uint32)
+    grp[::13] = np.iinfo(np.uint32).max
+    maps = []
+    for step in (5, 2):
+        gm = np.arange(ng, dtype=np.int32)
+        gm[::step] = -1
+        gm[gm >= 0] = np.arange((gm >= 0).sum(), dtype=np.int32)
+        maps.append(gm)
+    m = core.DeviceMatrix(indptr, idx, val, ng)
+    for gm in (maps[0], maps[1], maps[0]):
+        nv = int(gm.max()) + 1
+        cl = rng.uniform(0.5, 3.0, (G, nv)) if clip else None
+        got = resident(m, cm, gm, target, log, grp, G, nv, cl)
+        ref = [np.zeros((G, nv)) for _ in range(3)]
+        oracle.group_gene_sums(idx, val, cm, gm, target, log, None, indptr, 0, grp, *ref, cl)
+        np.testing.assert_allclose(got[0], ref[0], rtol=1e-12, atol=1e-12)
+        np.testing.assert_allclose(got[1], ref[1], rtol=1e-12, atol=1e-12)
+        assert np.array_equal(got[2], ref[2])
+    m.close()
+
+
+def test_resident_group_sums_of_very_many_genes():
+    """More genes than a shared-memory bit set of them holds (1.86 million)."""
+    ng, n = 1_900_000, 6
+    idx = np.sort(np.random.default_rng(1).choice(ng, (n, 50), replace=False), axis=1).astype(np.uint32)
+    idx[:, -1] = ng - 1
+    indptr = np.arange(n + 1, dtype=np.int64) * 50
+    val = np.tile(np.arange(1, 51, dtype=np.float32), n)
+    cm, gm = np.arange(n, dtype=np.int64), np.arange(ng, dtype=np.int32)
+    grp = (np.arange(n) % 2).astype(np.uint32)
+    m = core.DeviceMatrix(indptr, idx.ravel(), val, ng)
+    got = resident(m, cm, gm, 1e4, True, grp, 2, ng)
+    m.close()
+    ref = [np.zeros((2, ng)) for _ in range(3)]
+    oracle.group_gene_sums(idx.ravel(), val, cm, gm, 1e4, True, None, indptr, 0, grp, *ref)
+    np.testing.assert_allclose(got[0], ref[0], rtol=1e-12, atol=1e-12)
+    np.testing.assert_allclose(got[1], ref[1], rtol=1e-12, atol=1e-12)
+    assert np.array_equal(got[2], ref[2])
