@@ -330,14 +330,47 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
 // Bound by HBM and issue: 100,000 cells x 33,538 genes with 222 M entries
 // take 368 us (4.8 TB/s) against 925 for the gene ranges, whose windows of
 // ~130 entries each cost a reduction and two or three shared-memory adds per
-// entry; 2,700 cells with 2.3 M entries take 45 us against 91.  Gene maps
-// above the table's 46,479 genes keep the ranges.  One block loading ahead:
-// two spill (402 us); the adds themselves are hidden (the same time without
-// them).  60 M entries of which 0 / 2 / 20 % are 5000: 118 / 175 / 242 us
-// against 286; only a matrix of nothing but such values is slower (607).
+// entry; 2,700 cells with 2.3 M entries take 45 us against 91.  One block
+// loading ahead: two spill (402 us); the adds themselves are hidden (the same
+// time without them).
+//
+// The ranges stay for gene maps above the table's 46,479 genes and for
+// matrices with many values outside [0, 2048), whose global adds queue on the
+// genes' totals, the sooner the fewer genes there are.  Table against ranges:
+// 60 M entries over 33,000 genes 178 / 246 / 295 / 608 us at a share of 2 / 20 /
+// 40 / 100 % against 303; 40 M over 5,000 genes 119 / 128 / 203 us at 5 / 10 /
+// 20 % against 144; 8 M over 1,000 genes 42 / 56 / 397 us at 5 / 10 / 100 %
+// against 50; 6 M over 200 genes 47 / 93 us at 2 / 5 % against 68.  qc_few_large
+// keeps below these crossings.
 constexpr int kQcThreads = 1024;
 constexpr int kQcEpoch = 1023;
 constexpr uint32_t kQcSumMask = (1u << 22) - 1u;
+constexpr int kQcSamples = 65536;
+
+// *count += values outside [0, 2048) among kQcSamples of the matrix, one from
+// each of as many equal pieces at a hashed place (an even stride could meet
+// the same gene in every row); all of them when there are no more.
+__global__ void __launch_bounds__(256) k_count_large(const float *__restrict__ values, int64_t nnz, int *count) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t n = nnz < kQcSamples ? nnz : kQcSamples;
+    bool large = false;
+    if (i < n) {
+        const int64_t lo = i * nnz / n, width = (i + 1) * nnz / n - lo;
+        const float x = __ldg(values + lo + (int64_t)((uint32_t)i * 2654435761u) % width);
+        large = !(x >= 0.0f && x < 2048.0f);
+    }
+    const int in_block = __syncthreads_count(large);
+    if (threadIdx.x == 0 && in_block) atomicAdd(count, in_block);
+}
+
+int launch_count_large(const float *values, int64_t nnz, int *count, cudaStream_t st) {
+    if (nnz == 0) return CREST_OK;
+    k_count_large<<<kQcSamples / 256, 256, 0, st>>>(values, nnz, count);
+    CREST_CUDA_TRY(cudaGetLastError());
+    return CREST_OK;
+}
+double large_share(int large, int64_t nnz) { return large / (double)std::max<int64_t>(1, std::min<int64_t>(nnz, kQcSamples)); }
+static bool qc_few_large(double share, int64_t n_genes) { return share <= std::min(0.3, 0.02 + 8e-6 * (double)n_genes); }
 
 __host__ __device__ inline int64_t qc_slots(int64_t n_gene_map) { return round_up(n_gene_map + 1, 16); }
 
@@ -556,10 +589,10 @@ int sweep_ctas(int64_t n_spans, int64_t cell_cap) {
 }
 
 int launch_qc_sweep(const DevChunk &c, const RangeIndex &ix, const uint8_t *flag, uint32_t *gene_ncells,
-                    double *gene_total, const RowOut &row, bool strict, int *status, cudaStream_t st) {
+                    double *gene_total, const RowOut &row, bool strict, double large, int *status, cudaStream_t st) {
     if (c.n_spans == 0) return CREST_OK;
     const size_t table = (size_t)qc_slots(c.n_gene_map) * 5;
-    if (strict && table <= (size_t)kMaxSmem) {  // up to 46,479 genes
+    if (strict && qc_few_large(large, c.n_gene_map) && table <= (size_t)kMaxSmem) {  // up to 46,479 genes
         CREST_TRY(ensure_smem_attr((const void *)k_qc_table, table));
         prof::Scope ps("qc_csr", st);
         k_qc_table<<<sweep_ctas(c.n_spans, 0), kQcThreads, table, st>>>(c, flag, gene_ncells, gene_total, row, status);
@@ -572,7 +605,7 @@ int launch_qc_sweep(const DevChunk &c, const RangeIndex &ix, const uint8_t *flag
     const size_t smem = qc_sweep_smem(ix.log2_s, ceil_div(c.n_spans, ctas));
     CREST_REQUIRE(smem <= (size_t)kMaxSmem, CREST_EINVAL, "QC sweep: %zu B of shared memory", smem);
     CREST_TRY(ensure_smem_attr((const void *)k_qc_sweep, smem));
-    prof::Scope ps("qc_csr", st);
+    prof::Scope ps("qc_ranges_csr", st);
     k_qc_sweep<<<ctas, kSweepThreads, smem, st>>>(c, ix, flag, gene_ncells, gene_total, row, status);
     CREST_CUDA_TRY(cudaGetLastError());
     return CREST_OK;

@@ -63,11 +63,16 @@ constexpr int kSweepThreads = 768;
 int launch_range_index(const int64_t *indptr, const uint32_t *genes, int64_t n_cells, int log2_s, int n_ranges,
                        int32_t *off, int *unsorted, cudaStream_t st);
 // Per-gene QC sums and per-row (t, n, f) of a piece whose spans are matrix
-// cells first_cell + i.  strict: no row holds a gene id twice.  Integral
-// values only: bit 1 of *status is set otherwise and the results must be
-// discarded.
+// cells first_cell + i.  strict: no row holds a gene id twice; large: the
+// share of the values that the one-table form cannot hold in a word
+// (large_share).  Integral values only: bit 1 of *status is set otherwise and
+// the results must be discarded.
 int launch_qc_sweep(const DevChunk &c, const RangeIndex &ix, const uint8_t *flag, uint32_t *gene_ncells,
-                    double *gene_total, const RowOut &row, bool strict, int *status, cudaStream_t st);
+                    double *gene_total, const RowOut &row, bool strict, double large, int *status, cudaStream_t st);
+// *count += such values in a sample of a matrix's nnz values, and the share
+// that a count stands for.
+int launch_count_large(const float *values, int64_t nnz, int *count, cudaStream_t st);
+double large_share(int count, int64_t nnz);
 // gene_stats of a piece given its per-span kept-gene totals.
 int launch_gene_stats_sweep(const DevChunk &c, const RangeIndex &ix, const double *total, double *out,
                             cudaStream_t st);

@@ -97,3 +97,21 @@ def test_other_values(odd):
     for a, b in zip(got[:4], ref[:4]):
         assert np.array_equal(a, b)
     np.testing.assert_allclose(got[4], ref[4], rtol=1e-13)
+
+
+@pytest.mark.parametrize("n", [60, 40_000])
+@pytest.mark.parametrize("share,kernel", [(0.0, "qc_csr"), (0.01, "qc_csr"), (0.04, "qc_ranges_csr"), (1.0, "qc_ranges_csr")])
+def test_large_values_take_the_ranges(n, share, kernel):
+    """The table up to 2.8 % of values above 2047 at 1,000 genes, the gene ranges
+    beyond (a sample of up to 65,536 values decides, so shares to either side)."""
+    indptr, idx, val = rows(n, 1000, 200, 3)
+    every = int(1 / share) if share else 0
+    if every:
+        val[::every] = 5000.0
+    _lib.profile_enable(True)
+    got, ref = both(indptr, idx, val, 1000)
+    ran = _lib.profile_table()
+    _lib.profile_enable(False)
+    assert kernel in ran and {"qc_csr", "qc_ranges_csr"} & set(ran) == {kernel}
+    for a, b in zip(got, ref):
+        assert np.array_equal(a, b)
