@@ -1065,7 +1065,10 @@ __global__ void __launch_bounds__(1024) k_lanczos_step(double *V, int64_t d, int
 // keeps rows [r0, r1) of C in shared memory as FP32 (the run only brackets
 // the spectrum: FP32 products move the extreme Ritz values by ~1e-7
 // relative, far inside the guard the filter interval keeps) and the whole
-// current and previous vectors in FP64.  A step is one grid barrier: every
+// current vector in FP64; the previous one is in registers, each thread
+// holding the elements it updates, so that shared memory takes matrices of up
+// to 2,764 rows on 148 SMs (2,638 with both vectors there; larger ones take a
+// launch per step, 1.34 ms instead of 0.34 at 2,700 rows).  A step is one grid barrier: every
 // CTA publishes its rows of C v_j, then each reads the whole product and
 // forms alpha_j, v_{j+1} and beta_j for itself, in the same order everywhere.
 // The basis is not re-orthogonalised: that lets copies of converged extreme
@@ -1130,25 +1133,30 @@ struct LanczosArgs {
     int *err;
 };
 
-size_t lanczos_smem(int64_t d, int rows) { return sizeof(float) * (size_t)rows * d + sizeof(double) * 2 * (size_t)d; }
+constexpr int kLzThreads = 512, kLzHeld = 6;  // elements of the previous vector per thread, at most
 
-__global__ void __launch_bounds__(512) k_lanczos(LanczosArgs a) {
+size_t lanczos_smem(int64_t d, int rows) { return sizeof(float) * (size_t)rows * d + sizeof(double) * (size_t)d; }
+
+__global__ void __launch_bounds__(kLzThreads) k_lanczos(LanczosArgs a) {
     extern __shared__ __align__(16) unsigned char lz_smem[];
     __shared__ double red[32];
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
+    constexpr int nt = kLzThreads;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
     const int64_t d = a.d;
     const int64_t r0 = min(d, (int64_t)blockIdx.x * a.rows), r1 = min(d, r0 + a.rows);
     const int R = (int)(r1 - r0);
-    double *v = reinterpret_cast<double *>(lz_smem), *vp = v + d;  // v_j and v_{j-1}
-    float *cs = reinterpret_cast<float *>(vp + d);                 // rows x d: owned rows of C
+    double *v = reinterpret_cast<double *>(lz_smem);  // v_j
+    float *cs = reinterpret_cast<float *>(v + d);      // rows x d: owned rows of C
+    double vp[kLzHeld];                                // v_{j-1}: elements tid, tid + nt, ..
     for (int rr = 0; rr < R; ++rr)
         for (int64_t e = tid; e < d; e += nt) cs[rr * d + e] = (float)a.C[(r0 + rr) * a.ld + e];
     double s = 0.0;
     for (int64_t e = tid; e < d; e += nt) {
         v[e] = a.z0[e];
-        vp[e] = 0.0;
         s += v[e] * v[e];
     }
+#pragma unroll
+    for (int i = 0; i < kLzHeld; ++i) vp[i] = 0.0;
     double nrm = sqrt(block_sum(s, red));
     for (int64_t e = tid; e < d; e += nt) v[e] *= nrm > 0.0 ? 1.0 / nrm : 0.0;
     double beta = 0.0;
@@ -1174,17 +1182,24 @@ __global__ void __launch_bounds__(512) k_lanczos(LanczosArgs a) {
         for (int64_t e = tid; e < d; e += nt) s += v[e] * __ldcg(w + e);
         const double alpha = block_sum(s, red);
         s = 0.0;
-        for (int64_t e = tid; e < d; e += nt) {
-            const double z = __ldcg(w + e) - alpha * v[e] - beta * vp[e];
-            vp[e] = z;
+#pragma unroll
+        for (int i = 0; i < kLzHeld; ++i) {
+            const int64_t e = tid + i * nt;
+            if (e >= d) continue;
+            const double z = __ldcg(w + e) - alpha * v[e] - beta * vp[i];
+            vp[i] = z;
             s += z * z;
         }
         beta = sqrt(block_sum(s, red));
         const double inv = beta > 0.0 ? 1.0 / beta : 0.0;
-        for (int64_t e = tid; e < d; e += nt) vp[e] *= inv;
-        double *t = v;
-        v = vp;
-        vp = t;
+#pragma unroll
+        for (int i = 0; i < kLzHeld; ++i) {  // v_j and v_{j+1} change places
+            const int64_t e = tid + i * nt;
+            if (e >= d) continue;
+            const double t = v[e];
+            v[e] = vp[i] * inv;
+            vp[i] = t;
+        }
         if (blockIdx.x == 0 && tid == 0) {
             a.ab[j] = alpha;
             a.ab[kLanczos + j] = beta;
@@ -1262,12 +1277,12 @@ int lanczos_coop(EigWork &w, const double *C, int64_t d, int64_t ld, int L, cuda
     const int nb = (int)std::min<int64_t>(device_sms(), std::max<int64_t>(1, d / 4));
     const int rows = (int)ceil_div(d, nb);
     const size_t smem = lanczos_smem(d, rows);
-    if (smem > (size_t)kMaxSmem || ensure_smem_attr((const void *)k_lanczos, smem) != CREST_OK) {
+    if (d > kLzThreads * kLzHeld || smem > (size_t)kMaxSmem || ensure_smem_attr((const void *)k_lanczos, smem) != CREST_OK) {
         (void)cudaGetLastError();
         return CREST_ERUNTIME;
     }
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lanczos, 512, smem) != cudaSuccess || per_sm < 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lanczos, kLzThreads, smem) != cudaSuccess || per_sm < 1) {
         (void)cudaGetLastError();
         return CREST_ERUNTIME;
     }
@@ -1279,7 +1294,8 @@ int lanczos_coop(EigWork &w, const double *C, int64_t d, int64_t ld, int L, cuda
     LanczosArgs a{C, d, ld, L, rows, w.lz.as<double>(), w.lw.as<double>(), w.lab.as<double>(), w.lbar.as<unsigned>(),
                   w.fail.as<int>()};
     void *args[] = {&a};
-    if (cudaLaunchCooperativeKernel((const void *)k_lanczos, dim3(nb), dim3(512), args, smem, st) != cudaSuccess) {
+    prof::Scope ps("eig_lanczos", st);
+    if (cudaLaunchCooperativeKernel((const void *)k_lanczos, dim3(nb), dim3(kLzThreads), args, smem, st) != cudaSuccess) {
         (void)cudaGetLastError();
         return CREST_ERUNTIME;
     }
@@ -1487,14 +1503,12 @@ int eig_topk(const double *G, const double *colsum, int64_t d, int64_t n, int64_
         CREST_CUDA_TRY(cudaGetLastError());
         const int L = (int)std::min<int64_t>(kLanczos, d - 1);
         CREST_CUDA_TRY(cudaMemsetAsync(w.fail.ptr, 0, sizeof(int), st));
-        {
-            prof::Scope ps("eig_lanczos", st);
-            if (lanczos_coop(w, C, d, ld, L, st) != CREST_OK) {  // one launch per step, re-orthogonalised
-                k_cgs2<<<1, 1024, sizeof(double) * 64, st>>>(LZ, d, d, 0, 1, 1);
-                for (int j = 0; j < L; ++j) {
-                    k_symv<<<(unsigned)ceil_div(d * 32, 256), 256, 0, st>>>(C, d, ld, LZ + (int64_t)j * d, lw);
-                    k_lanczos_step<<<1, 1024, 0, st>>>(LZ, d, j, lw, lab);
-                }
+        if (lanczos_coop(w, C, d, ld, L, st) != CREST_OK) {  // one launch per step, re-orthogonalised
+            prof::Scope ps("eig_lanczos_steps", st);
+            k_cgs2<<<1, 1024, sizeof(double) * 64, st>>>(LZ, d, d, 0, 1, 1);
+            for (int j = 0; j < L; ++j) {
+                k_symv<<<(unsigned)ceil_div(d * 32, 256), 256, 0, st>>>(C, d, ld, LZ + (int64_t)j * d, lw);
+                k_lanczos_step<<<1, 1024, 0, st>>>(LZ, d, j, lw, lab);
             }
         }
         CREST_CUDA_TRY(cudaGetLastError());

@@ -12,7 +12,7 @@ the test's gaps are at least 1e-3, so 1e-7 with the square root of k terms."""
 import numpy as np
 import pytest
 
-from crest_b200 import _native
+from crest_b200 import _lib, _native
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +40,19 @@ def test_block_eigensolver_matches_lapack(d, k):
     assert np.linalg.norm(vecs - Q[:, :k] @ (Q[:, :k].T @ vecs), 2) <= 1e-7
     big = np.abs(vecs).argmax(0)
     assert np.all(vecs[big, np.arange(k)] > 0)
+
+
+@pytest.mark.parametrize("d,run", [(2639, "eig_lanczos"), (2764, "eig_lanczos"), (2765, "eig_lanczos_steps")])
+def test_spectrum_bounds_at_the_shared_memory_limit(d, run):
+    """The one-launch Lanczos run holds its rows and one vector in shared memory
+    up to 2,764 rows (148 SMs); one more takes a launch per step."""
+    k = 10
+    C, lam, Q = spectrum_case(d, k, d)
+    n = 5000
+    _lib.profile_enable(True)
+    vals, vecs, _ = _native.pca_from_gram(np.triu(C * (n - 1)), np.zeros(d), n, k)
+    ran = _lib.profile_table()
+    _lib.profile_enable(False)
+    assert run in ran and {"eig_lanczos", "eig_lanczos_steps"} & set(ran) == {run}
+    assert np.abs(vals - lam[:k]).max() <= 1e-10 * lam[0]
+    assert np.linalg.norm(vecs - Q[:, :k] @ (Q[:, :k].T @ vecs), 2) <= 1e-7
