@@ -81,18 +81,26 @@ int DevBuf::ensure(size_t bytes) {
         return CREST_ENOMEM;
     }
     cudaMemPool_t pool = device_pool();
-    cudaError_t e;
-    if (pool) {  // ordered on the legacy stream, which is idle here: usable on every stream after the sync
-        e = cudaMallocFromPoolAsync(&ptr, want, pool, 0);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-    } else {
-        e = cudaMalloc(&ptr, want);
-    }
+    auto take = [&] {
+        cudaError_t e;
+        if (pool) {  // ordered on the legacy stream, which is idle here: usable on every stream after the sync
+            e = cudaMallocFromPoolAsync(&ptr, want, pool, 0);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+        } else {
+            e = cudaMalloc(&ptr, want);
+        }
+        if (e != cudaSuccess) {
+            if (ptr && pool) cudaFreeAsync(ptr, 0);
+            ptr = nullptr;
+            cudaGetLastError();
+        }
+        return e;
+    };
+    cudaError_t e = take();
+    int dev = 0;
+    if (e == cudaErrorMemoryAllocation && cudaGetDevice(&dev) == cudaSuccess && tile_give_back(dev)) e = take();
     if (e != cudaSuccess) {
-        if (ptr && pool) cudaFreeAsync(ptr, 0);
-        ptr = nullptr;
         cap = 0;
-        cudaGetLastError();
         set_error("device allocation of %zu bytes failed: %s", want, cudaGetErrorString(e));
         return CREST_ENOMEM;
     }

@@ -61,11 +61,17 @@ inline int64_t tile_cells_default() {
     return round_up(v, 64);
 }
 
-// A Gram tile workspace sized for d genes.  The tile itself may live elsewhere
-// (`at`): passes over a resident or streamed matrix use one that the matrix
-// keeps, because a plan lasts for one PCA and giving 2 GB back to the pool and
-// taking it again per call cost 10 to 40 ms whenever a smaller buffer had
-// settled in its place (and two allocations even when not).
+// The Gram tile of a device's matrices (up to 4.3 GB at 2,000 genes): one,
+// lent to a pass and kept between passes, because a plan lasts for one PCA and
+// giving 2 GB back to the pool and taking it again per call cost 10 to 40 ms
+// whenever a smaller buffer had settled in its place (and two allocations even
+// when not).  A pass that finds it lent out has one of its own.
+// tile_give_back returns an idle tile to the pool and says whether there was
+// one: with the last matrix of the device, and when another allocation fails.
+bool tile_give_back(int device);
+
+// A Gram tile workspace sized for d genes; the tile itself may live elsewhere
+// (`at`).
 struct GramBufs {
     DevBuf tile, colsum_chunk, n_kept, shift, status, aux, colsum_part, parts;
     int ensure(GramWork &w, int64_t d, int precision, int64_t m_cap, DevBuf *at = nullptr) {
