@@ -30,9 +30,6 @@ int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st);
 int copy_out(void *host, const void *dev, size_t bytes, cudaStream_t st);
 template <class T>
 int add_out(double *host, const T *dev, int64_t n, cudaStream_t st);
-// The pinned buffers are given back when the last holder drops them.
-void staging_hold();
-void staging_drop();
 
 template <class T>
 inline int upload(DevBuf &b, const T *src, int64_t n, cudaStream_t st) {

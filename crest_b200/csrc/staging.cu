@@ -8,9 +8,12 @@
 // other threads, so the page faults and the copying spread over cores (98 MB of
 // a chunk's entries: 3.4 ms instead of 9.5; 40 MB of scores into a new array:
 // 2.6 to 4 ms instead of 8.8).  Threads live for the call only (nothing to hand
-// over a fork); a set of pinned buffers per device (12 MB) is kept between calls
-// and given back when the last matrix is freed.  A call that finds the buffers
-// in use by another thread, or cannot have them, copies as before.
+// over a fork).  The first large copy on a device takes 12 MB of pinned buffers
+// and the process keeps them, like the per-chunk workspaces: pinning them takes
+// 10 to 15 ms and giving them back 1.5, which a program that opens, reduces and
+// frees one matrix after another would otherwise pay for each.  A call that
+// finds the buffers in use by another thread, or cannot have them, copies as
+// before.
 #include <stdlib.h>
 #include <string.h>
 
@@ -58,7 +61,6 @@ struct Ring {
 };
 
 Ring g_ring[64];
-std::atomic<int> g_users{0};
 
 bool pageable(const void *p) {
     cudaPointerAttributes at;
@@ -202,22 +204,5 @@ int add_out(double *host, const T *dev, int64_t n, cudaStream_t st) {
 }
 template int add_out<double>(double *, const double *, int64_t, cudaStream_t);
 template int add_out<uint32_t>(double *, const uint32_t *, int64_t, cudaStream_t);
-
-void staging_hold() { g_users.fetch_add(1); }
-void staging_drop() {
-    if (g_users.fetch_sub(1) != 1) return;
-    int was = 0;
-    if (cudaGetDevice(&was) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    for (int d = 0; d < 64; ++d) {
-        std::unique_lock<std::mutex> lock(g_ring[d].mu, std::try_to_lock);
-        if (!lock.owns_lock() || !g_ring[d].ready) continue;
-        cudaSetDevice(d);
-        g_ring[d].release();
-    }
-    cudaSetDevice(was);
-}
 
 }  // namespace crest
