@@ -16,6 +16,8 @@
 // before.
 #include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <atomic>
 #include <mutex>
@@ -28,7 +30,15 @@ namespace crest {
 namespace {
 
 constexpr size_t kPiece = 1u << 20;     // 256 kB: the driver calls cost as much as the copies; 2 MB: no gain
-constexpr size_t kStageMin = 2u << 20;  // below, thread start-up (0.1 ms) costs what the threads save
+// Sizes from which the threads save more than they cost.  They find cold cores,
+// so a copy of a few MB takes 0.15 to 0.5 ms (both sides warm), where the plain
+// one takes 0.07 ms per MB; into pages that are not there yet the plain one
+// takes 0.45 ms per MB.  Plain against staged, in a Python process: in 2.3 / 3.8
+// / 5.3 / 12 MB 0.16 / 0.25 / 0.33 / 0.68 ms against 0.24 / 0.26 / 0.30 / 0.51;
+// QC's two sums out into warm arrays of 2.3 / 4.6 / 9.2 MB 0.94 / 1.65 / 3.2 ms
+// (whole call) against 1.4 / 2.4 / 3.2, into new ones 3.5 / 6.8 / 13.6 against
+// 2.6 / 4.3 / 6.5.
+constexpr size_t kStageIn = 5u << 20, kStageOutNew = 2u << 20, kStageOutWarm = 12u << 20;
 constexpr int kStageThreads = 6;        // 4 to 12 within 5 %
 constexpr int kSlots = 2 * kStageThreads;
 
@@ -71,6 +81,18 @@ bool pageable(const void *p) {
     return at.type == cudaMemoryTypeUnregistered;
 }
 
+// Whether most pages of a host array of less than kStageOutWarm bytes exist
+// (false when the system does not say).
+bool mostly_there(const void *p, size_t bytes) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE), a = (size_t)p / page * page;
+    const size_t n = ((size_t)p + bytes - a + page - 1) / page;
+    unsigned char there[kStageOutWarm / 4096 + 2];
+    if (n > sizeof there || mincore(reinterpret_cast<void *>(a), n * page, there) != 0) return false;
+    size_t have = 0;
+    for (size_t i = 0; i < n; ++i) have += there[i] & 1;
+    return 2 * have > n;
+}
+
 // body(t) for t < n on n threads, as many as can be had.
 template <class F>
 void on_threads(int n, F &&body) {
@@ -104,7 +126,7 @@ struct Share {
 // has to go the plain way.
 template <class F>
 bool in_pieces(const void *host, size_t bytes, cudaError_t &err, F &&work) {
-    if (bytes < kStageMin || !pageable(host)) return false;
+    if (!pageable(host)) return false;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
         cudaGetLastError();
@@ -135,7 +157,7 @@ bool in_pieces(const void *host, size_t bytes, cudaError_t &err, F &&work) {
 
 int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st) {
     cudaError_t err = cudaSuccess;
-    const bool done = in_pieces(host, bytes, err, [&](const Share &sh) {
+    const bool done = bytes >= kStageIn && in_pieces(host, bytes, err, [&](const Share &sh) {
         cudaError_t e = cudaSuccess;
         for (size_t i = 0; i < sh.count() && e == cudaSuccess; ++i) {
             e = cudaEventSynchronize(sh.ev[i & 1]);  // the buffer's transfer before
@@ -156,6 +178,7 @@ namespace {
 // Device data through the buffers into sink(pointer, offset, bytes); false: not taken.
 template <class F>
 bool drain(const void *host, const void *dev, size_t bytes, cudaStream_t st, cudaError_t &err, F &&sink) {
+    if (bytes < kStageOutNew || (bytes < kStageOutWarm && mostly_there(host, bytes))) return false;
     return in_pieces(host, bytes, err, [&](const Share &sh) {
         auto fetch = [&](size_t i) {
             cudaError_t e = cudaMemcpyAsync(sh.buf[i & 1], static_cast<const unsigned char *>(dev) + sh.at(i), sh.size(i),

@@ -2,6 +2,7 @@
 to those of small pieces (which take the plain copies), for sizes around the
 pieces and with two threads at once (one finds the buffers in use)."""
 
+import mmap
 import threading
 import time
 
@@ -91,3 +92,39 @@ def test_a_matrix_after_another_does_not_pay_for_the_buffers():
             times.append(time.perf_counter() - t)
         took[n] = min(times)
     assert took[7000] - took[1600] < 7e-3, took
+
+
+@pytest.mark.parametrize("n", [4369, 4370])  # 5,242,800 and 5,244,000 bytes an array: around 5 MB
+def test_copies_in_around_their_limit(n):
+    idx, val, indptr = chunk(n, n)
+    whole = sums(idx, val, indptr, n, [0, n])
+    parts = sums(idx, val, indptr, n, list(range(0, n, 500)) + [n])
+    for a, b in zip(whole, parts):
+        assert np.array_equal(a, b)
+    assert whole[2].sum() == len(idx)
+
+
+@pytest.mark.parametrize("n", [262_143, 262_144, 1_572_863, 1_572_864])  # 8 bytes each: around 2 and 12 MB
+@pytest.mark.parametrize("offset", [0, 8, 4088])
+def test_copies_out_into_new_and_warm_arrays(n, offset):
+    """Sums of every cell into pages that exist, that do not, and that are half
+    there, at any place in a page; bytes around them stay."""
+    indptr = np.arange(n + 1, dtype=np.int64)
+    val = (np.arange(n) % 1000 + 1).astype(np.float32)
+    m = core.DeviceMatrix(indptr, np.zeros(n, np.uint32), val, 1)
+    cm, gm, flag = np.arange(n, dtype=np.int64), np.zeros(1, np.int32), np.ones(1, np.uint8)
+    for touched in (0.0, 0.4, 1.0):
+        mem = [mmap.mmap(-1, 8 * n + 8192) for _ in range(2)]
+        for buf in mem:
+            np.frombuffer(buf, np.uint8)[:int(touched * len(buf))] = 7
+        whole = [np.frombuffer(buf, np.uint8) for buf in mem]
+        total, flagged = (w[offset:offset + 8 * n].view(np.float64) for w in whole)
+        ngenes, gn, gt = np.zeros(n, np.uint32), np.zeros(1, np.uint32), np.zeros(1)
+        _lib.call("crest_matrix_qc", m.handle, _lib.ptr(cm), _lib.ptr(gm), _lib.ptr(flag), n, 1, _lib.ptr(total),
+                  _lib.ptr(ngenes), _lib.ptr(flagged), _lib.ptr(gn), _lib.ptr(gt))
+        assert np.array_equal(total, val) and np.array_equal(flagged, val)
+        assert gn[0] == n and gt[0] == val.sum(dtype=np.float64)
+        for w in whole:
+            assert np.all(w[:offset] == (7 if touched else 0))
+            assert np.all(w[offset + 8 * n:] == (7 if touched == 1.0 else 0))
+    m.close()
