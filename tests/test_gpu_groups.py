@@ -203,3 +203,27 @@ def test_resident_group_sums_of_very_many_genes():
     np.testing.assert_allclose(got[0], ref[0], rtol=1e-12, atol=1e-12)
     np.testing.assert_allclose(got[1], ref[1], rtol=1e-12, atol=1e-12)
     assert np.array_equal(got[2], ref[2])
+
+
+@pytest.mark.parametrize("groups", [3, 436, 437, 900])  # 600 genes: up to and from 2 MB an array, more than one huge page
+@pytest.mark.parametrize("stats", [True, False])
+def test_group_sums_are_arrays_of_their_own(small_counts, groups, stats):
+    """Zero to begin with, writable, and none keeps another's memory alive."""
+    indptr, indices, data, n_genes = small_counts[:4]
+    bf = cb.BioFrame.from_csr(indptr, indices, data, n_genes, var=pd.DataFrame({"gene_name": small_counts[4]}))
+    grp = (np.arange(bf.n_obs) % groups).astype(np.uint32)
+    ref = [np.zeros((groups, n_genes)) for _ in range(3)]
+    oracle.group_gene_sums(indices, data, np.arange(bf.n_obs, dtype=np.int64), np.arange(n_genes, dtype=np.int32), 0.0,
+                           False, None, indptr, 0, grp, *ref)
+    got = cb.pp.group_gene_sums(bf, grp, groups, stats=stats)
+    got = got if stats else (got,)
+    for a, r in zip(got, ref):
+        assert a.flags.c_contiguous and a.flags.writeable and a.dtype == np.float64
+        assert np.array_equal(a, r)  # raw integer counts: exact
+        held = a
+        while isinstance(held, np.ndarray) and held.base is not None:
+            held = held.base
+        size = held.nbytes if isinstance(held, np.ndarray) else len(held)
+        assert size < a.nbytes + (1 << 21)
+    for i, a in enumerate(got):
+        assert not any(np.shares_memory(a, b) for b in got[i + 1:])
