@@ -18,7 +18,8 @@ import numpy as np
 import pytest
 
 import oracle
-from crest_b200 import _lib, _native
+from crest_b200 import _lib, _native, core
+from crest_b200.tl import PcaPlan
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +93,36 @@ def test_injected_allocation_failure():
     env = dict(os.environ, CREST_INJECT_ALLOC_FAIL="1")
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600, env=env)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr[-3000:]
+
+
+def test_gene_stats_after_a_pass_without_room(small_counts, monkeypatch):
+    """The N-th allocation of a Gram pass fails, N = 1, 2, ..: the pass reports
+    it or goes on without its compact form, and the gene statistics of the
+    matrix stay what they were (the gene-major copy that made room is built
+    again)."""
+    indptr, indices, data, cm, gm, sub, d = gram_case(small_counts)
+    ng = len(gm)
+
+    def stats(m):
+        out = np.zeros((ng, 5))
+        _lib.call("crest_matrix_gene_stats", m.handle, _lib.ptr(cm), _lib.ptr(gm), 1e4, 1, ng, _lib.ptr(out))
+        return out
+
+    gone_on = 0
+    for n in range(1, 25):
+        m, p = core.DeviceMatrix(indptr, indices, data, ng), PcaPlan(d, "fp64")
+        before = stats(m)
+        assert before[:, 4].sum() == len(indices)
+        monkeypatch.setenv("CREST_INJECT_ALLOC_FAIL", str(n))
+        try:
+            p.accumulate(m, cm, gm, 1e4, True, sub, ng, _lib.Scale(0, None, None, 0.0))
+            gone_on += 1
+        except _lib.CrestError as e:
+            assert f"status {_lib.ENOMEM}" in str(e)
+        monkeypatch.delenv("CREST_INJECT_ALLOC_FAIL")
+        after = stats(m)
+        assert np.array_equal(after[:, 4], before[:, 4])
+        np.testing.assert_allclose(after, before, rtol=1e-12)
+        p.close()
+        m.close()
+    assert gone_on >= 2
