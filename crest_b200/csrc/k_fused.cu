@@ -137,9 +137,9 @@ __device__ __forceinline__ void add_groups(double (&acc)[4]) {
 
 // Cells are spread one to a warp, or one to a block of kCellWarps warps that
 // take its 32-entry segments in turn: a warp needs about 5 us per segment, a
-// chain of loads and divisions, so with fewer cells than the chip has warps
-// the segments of a cell are the parallelism (512 cells x 175 entries: forward
-// 38 -> 10 us, entry pass of the backward 44 -> 14 us).
+// chain of loads and divisions, so with few cells the segments of a cell are
+// the parallelism (512 cells x 175 entries: forward 38 -> 10 us, entry pass of
+// the backward 44 -> 14 us).
 constexpr int kCellWarps = 8;
 
 template <int LPR, int WPC>
@@ -469,8 +469,20 @@ __global__ void k_to_float(const double *__restrict__ in, int64_t n, float *__re
     if (i < n) out[i] = (float)in[i];
 }
 
-// A block per cell while all cells' blocks are resident at once (four a SM).
+// A block per cell while all cells' blocks are resident at once (four a SM):
+// then it costs nothing even where a cell has one segment.  Beyond, it pays
+// where cells have several segments, which the backward knows (nnz): up to 64
+// cells an SM when they average 128 entries or more.  Warp against block per
+// cell, backward up to the W gradient: k = 50, 900 cells x 190 entries 52 against
+// 38 us, 4,736 x 190 153 / 114, 9,600 x 190 242 / 196, 9,600 x 128 174 / 151,
+// 20,000 x 128 302 / 280 but 229 / 259 at k = 100; 1,200 x 60 36 / 36, 2,400 x 60
+// 42 / 44, 2,400 x 20 31 / 43.  Forward: 592 x 190 28 / 15, 1,200 x 190 28 / 21,
+// 4,736 x 190 44 / 49, 600 x 20 17 / 20, 1,200 x 20 18 / 22: less to win and no
+// count of the entries at hand, so it keeps the first line.
 bool cell_per_block(int64_t n) { return n <= (int64_t)device_sms() * 4; }
+bool cell_per_block(int64_t n, int64_t nnz) {
+    return cell_per_block(n) || (n <= (int64_t)device_sms() * 64 && nnz >= 128 * n);
+}
 
 int grid_warps(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 8), device_sms() * 16)); }
 
@@ -494,9 +506,9 @@ struct FusedWork {
         else if ((kp) == 64) fn<16, wpc><<<(grid), 256, 0, (st)>>>(__VA_ARGS__); \
         else fn<32, wpc><<<(grid), 256, 0, (st)>>>(__VA_ARGS__);                 \
     } while (0)
-#define CREST_FUSED_CELLS(fn, kp, n, st, ...)                                                     \
+#define CREST_FUSED_CELLS(fn, kp, n, by_block, st, ...)                                           \
     do {                                                                                          \
-        if (cell_per_block(n)) CREST_FUSED_CELLS_W(fn, kp, kCellWarps, (unsigned)(n), st, __VA_ARGS__); \
+        if (by_block) CREST_FUSED_CELLS_W(fn, kp, kCellWarps, (unsigned)(n), st, __VA_ARGS__); \
         else CREST_FUSED_CELLS_W(fn, kp, 1, grid_warps(n), st, __VA_ARGS__);                      \
     } while (0)
 
@@ -567,7 +579,7 @@ extern "C" int crest_fused_forward(const int64_t *indptr, const int32_t *indices
         prof::Scope ps("fused_fwd", st);
         const int kp = padded_columns(k);
         CREST_TRY(pad_rows(W, d, k, kp, w.wpad, st));
-        CREST_FUSED_CELLS(k_fused_fwd, kp, n, st, a, w.wpad.as<float4>(), scores);
+        CREST_FUSED_CELLS(k_fused_fwd, kp, n, cell_per_block(n), st, a, w.wpad.as<float4>(), scores);
     }
     CREST_CUDA_TRY(cudaGetLastError());
     return bad_ids(w, a.bad, st);
@@ -624,8 +636,8 @@ extern "C" int crest_fused_backward(const int64_t *indptr, const int32_t *indice
         CREST_TRY(pad_rows(W, d, k, kp, w.wpad, st));
         CREST_TRY(pad_rows(grad_scores, n, k, kp, w.gpad, st));
         if (n > 0)
-            CREST_FUSED_CELLS(k_fused_bwd_entries, kp, n, st, a, w.wpad.as<float4>(), w.gpad.as<float4>(), grad_values,
-                              grad_sf, offsets, fill, by_gene);
+            CREST_FUSED_CELLS(k_fused_bwd_entries, kp, n, cell_per_block(n, nnz), st, a, w.wpad.as<float4>(),
+                              w.gpad.as<float4>(), grad_values, grad_sf, offsets, fill, by_gene);
         CREST_CUDA_TRY(cudaGetLastError());
     }
     if (d > 0) {

@@ -150,3 +150,16 @@ def test_no_genes(n, k):
         assert torch.all(scores == 0) and torch.all(gsf == 0)
         assert torch.all(gx[:n * entries] == 0)
         assert torch.all(torch.isnan(W))  # an output of no rows, and an input of none
+
+
+@pytest.mark.parametrize("n,per", [(593, 330.0), (9472, 330.0), (9473, 330.0), (700, 110.0), (600, 140.0)])
+def test_spread_of_the_backward_over_blocks(n, per):
+    """The backward takes a block per cell up to 9,472 cells (148 SMs) that
+    average 128 entries: both sides of either line; the tolerances of this file."""
+    c = make_case(n=n, d=600, k=20, max_value=10.0, seed=n, nnz_per_cell=per)
+    s_gpu, gx, gsf, gW = gpu_run(c)
+    s_ref, rx, rsf, rW = ref_run(c)
+    assert rel(s_gpu, s_ref) <= 1e-5
+    assert rel(gx, rx) <= 1e-4
+    assert rel(gsf, rsf) <= 1e-4
+    assert rel(gW, rW) <= 1e-4
