@@ -44,10 +44,16 @@ constexpr int kCscBlockCells = 128;
 constexpr int64_t kSegEntries = 2048;  // of a segment: 64 per lane of its warp
 constexpr int kTabCounts = 8;          // counts tabulated per cell, at most
 constexpr size_t kTabBytes = 32u << 20;
-// Counts 1 .. T of n_cells cells: as many as keep the table a quarter of L2.
+// Counts 1 .. T of n_cells cells: as many as keep the table a quarter of L2, or
+// none when those are fewer than four (above 524,288 cells): a warp then meets
+// an untabulated count in nearly every step and evaluates anyway.  Table against
+// none: 250,000 cells (8 counts, 100 M entries) 385 us / 869, 500,000 (4, 50 M)
+// 354 / 455, 700,000 (2, 70 M) 654 / 618, 1 M (2, 100 M) 902 / 852, 2 M (1, 200 M)
+// 1752 / 1662, 8 M (1, 96 M) 1240 / 891.
+constexpr int kTabLeast = 4;
 inline int tab_counts(int64_t n_cells) {
     const int64_t fit = (int64_t)(kTabBytes / sizeof(CellValue)) / std::max<int64_t>(n_cells, 1);
-    return (int)std::max<int64_t>(1, std::min<int64_t>(kTabCounts, fit));
+    return fit < kTabLeast ? 0 : (int)std::min<int64_t>(kTabCounts, fit);
 }
 
 // cells [c0, c1) of a block, one warp per cell: f(gene, value, cell)
@@ -209,7 +215,7 @@ __global__ void __launch_bounds__(kStatsThreads) k_gene_stats_csc(DevChunk c, co
                     const double scale = __ldg(cell_scale + cell[u]);
                     vf = transform_value(c, scale, x[u]);
                     ev = expm1((double)vf);
-                    use[u] = !(scale < 0.0);  // a cell whose factor is NaN is a kept one
+                    use[u] = use[u] && !(scale < 0.0);  // a cell whose factor is NaN is a kept one
                 } else {
                     use[u] = use[u] && ev != -2.0;
                 }
