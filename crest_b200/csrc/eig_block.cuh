@@ -22,6 +22,15 @@ struct EigOut {
     int ticket;   // blocks of k_apply_rot that have finished
 };
 
+// Whether value u of index j stands before value v of index i in descending
+// order, the lower index first among equals and NaN last: a total order, so
+// ranks by it are a permutation whatever the values are (by u > v alone every
+// NaN takes rank 0 and other places of the permutation stay unwritten).
+__device__ __forceinline__ bool stands_before(double u, int j, double v, int i) {
+    if (isnan(u) || isnan(v)) return !isnan(u) || (isnan(v) && j < i);
+    return u > v || (u == v && j < i);
+}
+
 // One Cholesky-QR pass on the active columns Ya = V[:, j0 ..) of a block
 // whose first j0 columns are orthonormal: from S = V^T Ya (p x q, ld p; its
 // first j0 rows T = Vl^T Ya, the rest the Gram matrix of Ya) the coefficients
@@ -341,7 +350,7 @@ __global__ void __launch_bounds__(kRrThreads) k_rr(const double *__restrict__ H,
         int rank = 0;
         for (int P = 0; P < n; ++P) {
             const int i = at(P);
-            if (i < q && (D[P] > v || (D[P] == v && i < tid))) ++rank;
+            if (i < q && stands_before(D[P], i, v, tid)) ++rank;
         }
         if (tid < q) {
             perm[tid] = rank;

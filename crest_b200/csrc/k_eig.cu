@@ -703,16 +703,14 @@ int jacobi(const double *A, int n_in, double *Vwork, double *V, double *vals, in
 
 // ------------------------------------------------- order + emit results
 // perm = indices of the n_in leading Jacobi values sorted descending
-// (ties: lower index first); one thread per candidate.
+// (ties: lower index first, NaN last); one thread per candidate.
 __global__ void k_rank(const double *vals, int n_in, int *perm, double *sorted) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_in) return;
     const double v = vals[i];
     int r = 0;
-    for (int j = 0; j < n_in; ++j) {
-        const double u = vals[j];
-        if (u > v || (u == v && j < i)) ++r;
-    }
+    for (int j = 0; j < n_in; ++j)
+        if (stands_before(vals[j], j, v, i)) ++r;
     perm[r] = i;
     sorted[r] = v;
 }

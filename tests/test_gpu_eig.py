@@ -56,3 +56,21 @@ def test_spectrum_bounds_at_the_shared_memory_limit(d, run):
     assert run in ran and {"eig_lanczos", "eig_lanczos_steps"} & set(ran) == {run}
     assert np.abs(vals - lam[:k]).max() <= 1e-10 * lam[0]
     assert np.linalg.norm(vecs - Q[:, :k] @ (Q[:, :k].T @ vecs), 2) <= 1e-7
+
+
+@pytest.mark.parametrize("d,k", [(2, 2), (37, 37), (160, 160), (160, 50)])
+def test_nan_covariance_ranks_stay_a_permutation(d, k):
+    """With a NaN off the diagonal no rotation is taken (its threshold is NaN),
+    so the values are the diagonal: descending, ties by index, NaN last (and
+    reported as 0 like a negative one), each with its own unit vector.  The
+    ranks index the vectors, so they have to be a permutation."""
+    rng = np.random.default_rng(d)
+    diag = rng.integers(1, 1 + d // 3 + 1, d).astype(np.float64)
+    if d > 2:
+        diag[[3, d // 2, d - 2]] = np.nan
+    G = np.diag(diag)
+    G[0, 1] = np.nan
+    vals, vecs, _ = _native.pca_from_gram(G, np.zeros(d), 2, k)
+    order = sorted(range(d), key=lambda i: (np.isnan(diag[i]), -diag[i] if diag[i] == diag[i] else 0.0, i))[:k]
+    assert np.array_equal(vals, np.nan_to_num(diag[order], nan=0.0))
+    assert np.array_equal(vecs, np.eye(d)[:, order])
