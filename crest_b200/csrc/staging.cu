@@ -32,13 +32,16 @@ namespace {
 constexpr size_t kPiece = 1u << 20;     // 256 kB: the driver calls cost as much as the copies; 2 MB: no gain
 // Sizes from which the threads save more than they cost.  They find cold cores,
 // so a copy of a few MB takes 0.15 to 0.5 ms (both sides warm), where the plain
-// one takes 0.07 ms per MB; into pages that are not there yet the plain one
-// takes 0.45 ms per MB.  Plain against staged, in a Python process: in 2.3 / 3.8
-// / 5.3 / 12 MB 0.16 / 0.25 / 0.33 / 0.68 ms against 0.24 / 0.26 / 0.30 / 0.51;
+// one takes 0.07 ms per MB (less when the caller has just written the data, as
+// zeroed accumulators are); out into pages that are not there yet the plain one
+// takes 0.45 ms per MB.  Plain against staged, in a Python process: two arrays
+// in of 8 / 12 / 16 / 24 MB 1.17 / 1.59 / 2.05 / 3.13 ms (whole call) against
+// 1.04 / 1.28 / 1.56 / 2.06, one of them zeroed just before 5 / 8 / 12 / 16 / 24
+// MB 1.01 / 1.43 / 1.96 / 2.51 / 4.64 against 1.35 / 1.83 / 2.38 / 2.55 / 3.53;
 // QC's two sums out into warm arrays of 2.3 / 4.6 / 9.2 MB 0.94 / 1.65 / 3.2 ms
-// (whole call) against 1.4 / 2.4 / 3.2, into new ones 3.5 / 6.8 / 13.6 against
-// 2.6 / 4.3 / 6.5.
-constexpr size_t kStageIn = 5u << 20, kStageOutNew = 2u << 20, kStageOutWarm = 12u << 20;
+// against 1.4 / 2.4 / 3.2, into new ones 3.5 / 6.8 / 13.6 against 2.6 / 4.3 /
+// 6.5.
+constexpr size_t kStageIn = 16u << 20, kStageOutNew = 2u << 20, kStageOutWarm = 12u << 20;
 constexpr int kStageThreads = 6;        // 4 to 12 within 5 %
 constexpr int kSlots = 2 * kStageThreads;
 

@@ -128,3 +128,29 @@ def test_copies_out_into_new_and_warm_arrays(n, offset):
             assert np.all(w[:offset] == (7 if touched else 0))
             assert np.all(w[offset + 8 * n:] == (7 if touched == 1.0 else 0))
     m.close()
+
+
+@pytest.mark.parametrize("n", [4_194_303, 4_194_304, 4_456_449])  # 4 bytes each: around 16 MB, a ragged last piece
+def test_copies_in_from_untouched_pages(n):
+    """Values in pages that nothing has written (zeros), a third of them
+    written, and all of them: the sums over every 300th gene of 64 cells."""
+    cells = 64
+    indptr = np.linspace(0, n, cells + 1).astype(np.int64)
+    idx = np.concatenate([np.arange(k, dtype=np.uint32) for k in np.diff(indptr)])
+    n_genes = int(idx.max()) + 1
+    gm = np.full(n_genes, -1, np.int32)
+    gm[::300] = np.arange(len(gm[::300]))
+    nv = int(gm.max()) + 1
+    cm, flag = np.arange(cells, dtype=np.int64), np.zeros(nv, np.uint8)
+    for written in (0.0, 0.3, 1.0):
+        val = np.frombuffer(mmap.mmap(-1, 4 * n), np.float32)
+        val[:int(written * n)] = np.arange(int(written * n)) % 97 + 1
+        m = core.DeviceMatrix(indptr, idx, val, n_genes)
+        total, ngenes, flagged = np.zeros(cells), np.zeros(cells, np.uint32), np.zeros(cells)
+        gn, gt = np.zeros(nv, np.uint32), np.zeros(nv)
+        _lib.call("crest_matrix_qc", m.handle, _lib.ptr(cm), _lib.ptr(gm), _lib.ptr(flag), cells, nv, _lib.ptr(total),
+                  _lib.ptr(ngenes), _lib.ptr(flagged), _lib.ptr(gn), _lib.ptr(gt))
+        m.close()
+        kept = np.where(gm[idx] >= 0, val, 0.0).astype(np.float64)
+        assert np.array_equal(total, np.add.reduceat(kept, indptr[:-1]))
+        assert np.array_equal(gt, np.bincount(gm[idx][gm[idx] >= 0], val[gm[idx] >= 0], minlength=nv))
