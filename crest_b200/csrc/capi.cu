@@ -594,14 +594,16 @@ int crest_group_gene_sums(const crest_chunk *chunk, const uint32_t *group_of_row
     }
     CREST_TRY(zeros<double>(x->out0, ne, st));
     if (sumsq) CREST_TRY(zeros<double>(x->out1, ne, st));
-    if (nnz) CREST_TRY(zeros<uint32_t>(x->out2, ne, st));
+    const bool narrow = ne >= kNarrowCounts;
+    if (nnz) CREST_TRY(narrow ? zeros<uint32_t>(x->out2, ne, st) : zeros<double>(x->out2, ne, st));
     CREST_TRY(launch_group_gene_sums(dc, x->out5.as<uint32_t>(), n_vars, dclip, x->out0.as<double>(),
-                                     sumsq ? x->out1.as<double>() : nullptr, nnz ? x->out2.as<uint32_t>() : nullptr,
+                                     sumsq ? x->out1.as<double>() : nullptr, nnz ? x->out2.ptr : nullptr, narrow,
                                      st));
     CREST_CUDA_TRY(cudaStreamSynchronize(st));  // a failed pass leaves the caller's sums as they are
     CREST_TRY(add_out(sum, x->out0.as<double>(), ne, st));
     if (sumsq) CREST_TRY(add_out(sumsq, x->out1.as<double>(), ne, st));
-    if (nnz) CREST_TRY(add_out(nnz, x->out2.as<uint32_t>(), ne, st));
+    if (nnz && narrow) CREST_TRY(add_out(nnz, x->out2.as<uint32_t>(), ne, st));
+    if (nnz && !narrow) CREST_TRY(add_out(nnz, x->out2.as<double>(), ne, st));
     return CREST_OK;
 }
 

@@ -46,9 +46,12 @@ int launch_gene_stats_csc(const DevChunk &c, CscMatrix &m, const double *total, 
 
 // Exact k nearest neighbours (self excluded) of the rows of X (n x d f32, device).
 int launch_knn(const float *X, int64_t n, int d, int k, DevBuf &work, uint32_t *idx, float *dist, cudaStream_t st);
-// Per (group, var) sums of the transformed values (sumsq / nnz / clip may be NULL).
+// Per (group, var) sums of the transformed values (sumsq / nnz / clip may be
+// NULL); nnz in 32-bit integers when narrow (from kNarrowCounts pairs on), else
+// in doubles.
+constexpr int64_t kNarrowCounts = 65536;
 int launch_group_gene_sums(const DevChunk &c, const uint32_t *group_of_row, int64_t n_vars, const double *clip,
-                           double *sum, double *sumsq, uint32_t *nnz, cudaStream_t st);
+                           double *sum, double *sumsq, void *nnz, bool narrow, cudaStream_t st);
 // Gene-range index of a device-resident CSR matrix with rows sorted by gene
 // id: off[cell * (n_ranges - 1) + b - 1] = first entry of the row (relative
 // to its start) with gene >= b << log2_s, b = 1 .. n_ranges - 1.

@@ -227,3 +227,33 @@ def test_group_sums_are_arrays_of_their_own(small_counts, groups, stats):
         assert size < a.nbytes + (1 << 21)
     for i, a in enumerate(got):
         assert not any(np.shares_memory(a, b) for b in got[i + 1:])
+
+
+@pytest.mark.parametrize("groups,genes", [(1, 65_535), (3, 21_845), (4, 16_384), (2, 32_769), (1, 7)])
+def test_group_counts_around_their_narrow_form(groups, genes):
+    """Up to 65,535 pairs the counts are kept as wide as the sums, from 65,536
+    on in 32 bits: the same whole numbers either way, added to what the caller
+    holds, on a resident matrix and in chunks."""
+    rng = np.random.default_rng(genes)
+    n, per = 300, 7
+    idx = np.sort(np.stack([rng.choice(genes, per, replace=False) for _ in range(n)]), axis=1).astype(np.uint32).ravel()
+    indptr = np.arange(n + 1, dtype=np.int64) * per
+    val = rng.integers(1, 40, len(idx)).astype(np.float32)
+    cm, gm = np.arange(n, dtype=np.int64), np.arange(genes, dtype=np.int32)
+    grp = rng.integers(0, groups, n).astype(np.uint32)
+    ref = [np.full((groups, genes), 2.0) for _ in range(3)]
+    oracle.group_gene_sums(idx, val, cm, gm, 1e4, True, None, indptr, 0, grp, *ref)
+    m = core.DeviceMatrix(indptr, idx, val, genes)
+    kept = [np.full((groups, genes), 2.0) for _ in range(3)]
+    _lib.call("crest_matrix_group_gene_sums", m.handle, _lib.ptr(cm), _lib.ptr(gm), 1e4, 1, _lib.ptr(grp), n, groups,
+              genes, None, *[_lib.ptr(a) for a in kept])
+    m.close()
+    chunk = [np.full((groups, genes), 2.0) for _ in range(3)]
+    _native.group_gene_sums(idx, val, cm, gm, 1e4, True, None, indptr, 0, grp, *chunk)
+    totals = np.full((groups, genes), 2.0)
+    _native.group_gene_totals(idx, val, cm, gm, 1e4, True, None, indptr, 0, grp, totals)
+    for got in (kept, chunk):
+        np.testing.assert_allclose(got[0], ref[0], rtol=1e-12)
+        np.testing.assert_allclose(got[1], ref[1], rtol=1e-12)
+        assert np.array_equal(got[2], ref[2])
+    np.testing.assert_allclose(totals, ref[0], rtol=1e-12)
