@@ -599,11 +599,9 @@ int crest_group_gene_sums(const crest_chunk *chunk, const uint32_t *group_of_row
     CREST_TRY(launch_group_gene_sums(dc, x->out5.as<uint32_t>(), n_vars, dclip, x->out0.as<double>(),
                                      sumsq ? x->out1.as<double>() : nullptr, nnz ? x->out2.ptr : nullptr, narrow,
                                      st));
+    AddOut outs[3] = {{sum, x->out0.ptr, ne}, {sumsq, x->out1.ptr, ne}, {nnz, x->out2.ptr, ne, narrow}};
     CREST_CUDA_TRY(cudaStreamSynchronize(st));  // a failed pass leaves the caller's sums as they are
-    CREST_TRY(add_out(sum, x->out0.as<double>(), ne, st));
-    if (sumsq) CREST_TRY(add_out(sumsq, x->out1.as<double>(), ne, st));
-    if (nnz && narrow) CREST_TRY(add_out(nnz, x->out2.as<uint32_t>(), ne, st));
-    if (nnz && !narrow) CREST_TRY(add_out(nnz, x->out2.as<double>(), ne, st));
+    for (AddOut &o : outs) CREST_TRY(o.add(st));
     return CREST_OK;
 }
 

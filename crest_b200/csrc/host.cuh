@@ -4,6 +4,7 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "kernels.cuh"
 
@@ -24,12 +25,28 @@ inline int require_device() {
 // Copies of host arrays, pageable or pinned (staging.cu): large pageable ones
 // go through pinned buffers by several threads, others as cudaMemcpyAsync on
 // st.  copy_in may return before the transfer, with the source free to change
-// unless it is pinned; after copy_out or add_out the host data is complete
-// once st has been synchronised.  add_out: host[i] += dev[i].
+// unless it is pinned; after copy_out the host data is complete once st has
+// been synchronised.
 int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st);
 int copy_out(void *host, const void *dev, size_t bytes, cudaStream_t st);
-template <class T>
-int add_out(double *host, const T *dev, int64_t n, cudaStream_t st);
+
+// host[i] += dev[i] for n doubles, or 32-bit integers when narrow (nothing when
+// host is NULL).  Made while the device still works on dev: the plain way's
+// buffer, whose new pages cost as much as the copy, is then had meanwhile.
+class AddOut {
+  public:
+    AddOut(double *host, const void *dev, int64_t n, bool narrow = false);
+    int add(cudaStream_t st);  // dev is complete; so is host afterwards
+
+  private:
+    template <class T>
+    int add_as(cudaStream_t st);
+    double *host_;
+    const void *dev_;
+    int64_t n_;
+    bool narrow_, stage_;
+    std::vector<unsigned char> buf_;
+};
 
 template <class T>
 inline int upload(DevBuf &b, const T *src, int64_t n, cudaStream_t st) {

@@ -40,8 +40,11 @@ constexpr size_t kPiece = 1u << 20;     // 256 kB: the driver calls cost as much
 // MB 1.01 / 1.43 / 1.96 / 2.51 / 4.64 against 1.35 / 1.83 / 2.38 / 2.55 / 3.53;
 // QC's two sums out into warm arrays of 2.3 / 4.6 / 9.2 MB 0.94 / 1.65 / 3.2 ms
 // against 1.4 / 2.4 / 3.2, into new ones 3.5 / 6.8 / 13.6 against 2.6 / 4.3 /
-// 6.5.
-constexpr size_t kStageIn = 16u << 20, kStageOutNew = 2u << 20, kStageOutWarm = 12u << 20;
+// 6.5.  Sums added to the caller's (AddOut) go through the threads whatever the
+// pages: group sums of three warm arrays of 3.2 / 5.4 / 6.4 / 10.7 MB 4.4 / 4.3 /
+// 8.5 / 7.5 ms against 2.4 / 2.6 / 2.7 / 3.0.
+constexpr size_t kStageIn = 16u << 20, kStageOutNew = 2u << 20, kStageOutWarm = 12u << 20,
+                 kStageAdd = 2u << 20;
 constexpr int kStageThreads = 6;        // 4 to 12 within 5 %
 constexpr int kSlots = 2 * kStageThreads;
 
@@ -178,10 +181,13 @@ int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st) {
 }
 
 namespace {
+bool stage_out(const void *host, size_t bytes) {
+    return bytes >= kStageOutNew && (bytes >= kStageOutWarm || !mostly_there(host, bytes));
+}
+
 // Device data through the buffers into sink(pointer, offset, bytes); false: not taken.
 template <class F>
 bool drain(const void *host, const void *dev, size_t bytes, cudaStream_t st, cudaError_t &err, F &&sink) {
-    if (bytes < kStageOutNew || (bytes < kStageOutWarm && mostly_there(host, bytes))) return false;
     return in_pieces(host, bytes, err, [&](const Share &sh) {
         auto fetch = [&](size_t i) {
             cudaError_t e = cudaMemcpyAsync(sh.buf[i & 1], static_cast<const unsigned char *>(dev) + sh.at(i), sh.size(i),
@@ -202,33 +208,46 @@ bool drain(const void *host, const void *dev, size_t bytes, cudaStream_t st, cud
 
 int copy_out(void *host, const void *dev, size_t bytes, cudaStream_t st) {
     cudaError_t err = cudaSuccess;
-    if (!drain(host, dev, bytes, st, err, [&](const unsigned char *p, size_t at, size_t n) {
-            memcpy(static_cast<unsigned char *>(host) + at, p, n);
-        }))
+    const bool staged = stage_out(host, bytes) &&
+                        drain(host, dev, bytes, st, err, [&](const unsigned char *p, size_t at, size_t n) {
+                            memcpy(static_cast<unsigned char *>(host) + at, p, n);
+                        });
+    if (!staged)
         err = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
     CREST_CUDA_TRY(err);
     return CREST_OK;
 }
 
+AddOut::AddOut(double *host, const void *dev, int64_t n, bool narrow)
+    : host_(host), dev_(dev), n_(host && n > 0 ? n : 0), narrow_(narrow),
+      stage_((narrow ? sizeof(uint32_t) : sizeof(double)) * (size_t)n_ >= kStageAdd) {
+    if (!stage_) buf_.resize((narrow ? sizeof(uint32_t) : sizeof(double)) * (size_t)n_);
+}
+
 template <class T>
-int add_out(double *host, const T *dev, int64_t n, cudaStream_t st) {
-    if (n <= 0) return CREST_OK;
+int AddOut::add_as(cudaStream_t st) {
+    const size_t bytes = sizeof(T) * (size_t)n_;
     cudaError_t err = cudaSuccess;
-    if (drain(host, dev, sizeof(T) * (size_t)n, st, err, [&](const unsigned char *p, size_t at, size_t bytes) {
-            const T *v = reinterpret_cast<const T *>(p);
-            double *o = host + at / sizeof(T);
-            for (size_t i = 0; i < bytes / sizeof(T); ++i) o[i] += (double)v[i];
+    auto sum = [this](const T *v, size_t first, size_t n) {
+        double *o = host_ + first;
+        for (size_t i = 0; i < n; ++i) o[i] += (double)v[i];
+    };
+    if (stage_ && drain(host_, dev_, bytes, st, err, [&](const unsigned char *p, size_t at, size_t n) {
+            sum(reinterpret_cast<const T *>(p), at / sizeof(T), n / sizeof(T));
         })) {
         CREST_CUDA_TRY(err);
         return CREST_OK;
     }
-    std::vector<T> h(n);
-    CREST_CUDA_TRY(cudaMemcpyAsync(h.data(), dev, sizeof(T) * (size_t)n, cudaMemcpyDeviceToHost, st));
+    buf_.resize(bytes);  // when the pinned buffers were not to be had
+    CREST_CUDA_TRY(cudaMemcpyAsync(buf_.data(), dev_, bytes, cudaMemcpyDeviceToHost, st));
     CREST_CUDA_TRY(cudaStreamSynchronize(st));
-    for (int64_t i = 0; i < n; ++i) host[i] += (double)h[i];
+    sum(reinterpret_cast<const T *>(buf_.data()), 0, (size_t)n_);
     return CREST_OK;
 }
-template int add_out<double>(double *, const double *, int64_t, cudaStream_t);
-template int add_out<uint32_t>(double *, const uint32_t *, int64_t, cudaStream_t);
+
+int AddOut::add(cudaStream_t st) {
+    if (n_ == 0) return CREST_OK;
+    return narrow_ ? add_as<uint32_t>(st) : add_as<double>(st);
+}
 
 }  // namespace crest
