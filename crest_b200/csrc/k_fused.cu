@@ -64,9 +64,12 @@ __device__ __forceinline__ double fused_value(const FusedArgs &a, int32_t g, flo
 // 32 / LPR entries at a time, four columns per lane.  The copy has a row 0
 // even when there are no rows (d = 0): slots without an entry, and entries
 // whose gene id is outside [0, d), load that row and drop what they load.
+// The launch also clears the call's flag (`clear`, when it has no other fill):
+// a fill of its own costs a small call 2 us.
 __global__ void k_pad_rows(const float *__restrict__ in, int64_t rows, int64_t rows_out, int k, int kp,
-                           float *__restrict__ out) {
+                           float *__restrict__ out, int *clear) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0 && clear) *clear = 0;
     if (i >= rows_out * kp) return;
     const int64_t r = i / kp;
     const int j = (int)(i - r * kp);
@@ -514,10 +517,11 @@ struct FusedWork {
 
 int padded_columns(int64_t k) { return k <= 32 ? 32 : k <= 64 ? 64 : 128; }
 
-int pad_rows(const float *in, int64_t rows, int64_t k, int kp, DevBuf &buf, cudaStream_t st) {
+int pad_rows(const float *in, int64_t rows, int64_t k, int kp, DevBuf &buf, cudaStream_t st, int *clear = nullptr) {
     const int64_t rows_out = std::max<int64_t>(rows, 1);
     CREST_TRY(buf.ensure(sizeof(float) * (size_t)(rows_out * kp)));
-    k_pad_rows<<<(unsigned)ceil_div(rows_out * kp, 256), 256, 0, st>>>(in, rows, rows_out, (int)k, kp, buf.as<float>());
+    k_pad_rows<<<(unsigned)ceil_div(rows_out * kp, 256), 256, 0, st>>>(in, rows, rows_out, (int)k, kp, buf.as<float>(),
+                                                                          clear);
     CREST_CUDA_TRY(cudaGetLastError());
     return CREST_OK;
 }
@@ -525,14 +529,6 @@ int pad_rows(const float *in, int64_t rows, int64_t k, int kp, DevBuf &buf, cuda
 FusedWork &fused_work(int dev) {
     static thread_local FusedWork ws[64];
     return ws[dev];
-}
-
-// Flag buffer of the current device, cleared; its value is read by bad_ids().
-int arm_flag(FusedWork &w, FusedArgs &a, cudaStream_t st) {
-    CREST_TRY(w.bad.ensure(sizeof(int)));
-    CREST_CUDA_TRY(cudaMemsetAsync(w.bad.ptr, 0, sizeof(int), st));
-    a.bad = w.bad.as<int>();
-    return CREST_OK;
 }
 
 int bad_ids(FusedWork &w, const int *flag, cudaStream_t st) {
@@ -574,11 +570,12 @@ extern "C" int crest_fused_forward(const int64_t *indptr, const int32_t *indices
     CREST_TRY(current_device(&dev));
     FusedWork &w = fused_work(dev);
     cudaStream_t st = cudaStreamPerThread;
-    CREST_TRY(arm_flag(w, a, st));
+    CREST_TRY(w.bad.ensure(sizeof(int)));
+    a.bad = w.bad.as<int>();
     {
         prof::Scope ps("fused_fwd", st);
         const int kp = padded_columns(k);
-        CREST_TRY(pad_rows(W, d, k, kp, w.wpad, st));
+        CREST_TRY(pad_rows(W, d, k, kp, w.wpad, st, a.bad));
         CREST_FUSED_CELLS(k_fused_fwd, kp, n, cell_per_block(n), st, a, w.wpad.as<float4>(), scores);
     }
     CREST_CUDA_TRY(cudaGetLastError());

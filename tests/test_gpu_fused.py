@@ -163,3 +163,27 @@ def test_spread_of_the_backward_over_blocks(n, per):
     assert rel(gx, rx) <= 1e-4
     assert rel(gsf, rsf) <= 1e-4
     assert rel(gW, rW) <= 1e-4
+
+
+@pytest.mark.parametrize("n,k", [(3, 1), (700, 50)])
+def test_rejected_call_leaves_no_trace(n, k):
+    """The flag of an out-of-range gene id is the next call's again: rejected,
+    accepted with the right scores, rejected, forward and backward."""
+    rng = np.random.default_rng(n)
+    dev, d, per = torch.device("cuda"), 30, 40
+    indptr = torch.arange(n + 1, device=dev) * per
+    good = torch.from_numpy(rng.integers(0, d, n * per).astype(np.int32)).to(dev)
+    bad = good.clone()
+    bad[-1] = d
+    v = torch.ones(n * per, device=dev, requires_grad=True)
+    sf = torch.full((n,), 2.0, device=dev, requires_grad=True)
+    W = torch.ones((d, k), device=dev, requires_grad=True)
+    mean, std = torch.zeros(d, dtype=torch.float64, device=dev), torch.ones(d, dtype=torch.float64, device=dev)
+    want = per * np.log1p(0.5)
+    for _ in range(2):
+        with pytest.raises(Exception, match="gene ids"):
+            fused_scale_project(v, sf, W, indptr, bad, mean, std, 10.0)
+        s = fused_scale_project(v, sf, W, indptr, good, mean, std, 10.0)
+        assert torch.allclose(s, torch.full_like(s, want), rtol=1e-6)
+        g = torch.autograd.grad(s.sum(), (v, sf, W))
+        assert torch.allclose(g[0], torch.full_like(g[0], k / 3.0), rtol=1e-6)
