@@ -495,18 +495,57 @@ __host__ __device__ inline int64_t syrk_owner(int64_t unit, int64_t units, int64
     return ((unit + 1) * ctas - 1) / units;
 }
 
+// CTAs of a launch.  Even runs leave parts of tiles to be written, read and
+// added in a second launch, the more the more tiles there are: with one CTA per
+// SM about as long as kPartsGroups x tiles / SMs groups take.  A CTA per tile is
+// taken where it is longer than even runs by no more than that (no tile is then
+// in parts, nor when whole tiles come out even).  Even runs against a CTA per
+// tile: 2,000 genes (136 tiles), 64 / 384 / 1,024 / 2,048 cells 34 / 73 / 130 /
+// 227 us against 23 / 56 / 123 / 229; 1,501 (78), 64 / 192 / 256 / 512 cells 34 /
+// 39 / 42 / 56 against 23 / 36 / 43 / 70; 1,000 (36), 64 / 128 cells 20 / 22
+// against 22 / 29.
+constexpr int64_t kPartsGroups = 6;
+inline int64_t syrk_ctas(int64_t tiles, int64_t groups, int64_t sms) {
+    if (tiles <= sms && groups * (sms - tiles) <= kPartsGroups * tiles) return tiles;
+    return std::min(sms, tiles * groups);
+}
+
 // Row / column of this thread's output (p, q) in a tile.
 __device__ __forceinline__ int syrk_row(int tid, int p) { return (p < 4 ? 0 : 60) + (tid >> 4) * 4 + p; }
 __device__ __forceinline__ int syrk_col(int tid, int q) { return (q < 4 ? 0 : 60) + (tid & 15) * 4 + q; }
 
-__device__ __forceinline__ void syrk_add(double v, int64_t a, int64_t b, int64_t d, const double *shift,
-                                         const double *colsum_c, double nk, double *G) {
-    if (a >= d || b >= d || b < a) return;
-    if (shift) {
-        const double ba = shift[a], ca = colsum_c[a], bb = shift[b], cb = colsum_c[b];
-        v = v - ba * cb - ca * bb - nk * ba * bb;
+// The column side of the shift correction, and one row of outputs into G with
+// it: the loads of a row go out together (one after another, each behind the
+// store of the element before, the 64 outputs of a thread took 5 to 12 us more).
+struct SyrkCols {
+    double shift[8], colsum[8];
+};
+__device__ __forceinline__ void syrk_cols(SyrkCols &c, int64_t b0, int tid, int64_t d, const double *shift,
+                                          const double *colsum_c) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int64_t b = b0 + syrk_col(tid, q);
+        c.shift[q] = shift && b < d ? __ldg(shift + b) : 0.0;
+        c.colsum[q] = shift && b < d ? __ldg(colsum_c + b) : 0.0;
     }
-    G[a * d + b] += v;
+}
+__device__ __forceinline__ void syrk_add_row(const double (&v)[8], const SyrkCols &c, int64_t a, int64_t b0, int tid,
+                                             int64_t d, const double *shift, const double *colsum_c, double nk,
+                                             double *G) {
+    if (a >= d) return;
+    const double ba = shift ? __ldg(shift + a) : 0.0, ca = shift ? __ldg(colsum_c + a) : 0.0;
+    double g[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int64_t b = b0 + syrk_col(tid, q);
+        g[q] = b < d && b >= a ? G[a * d + b] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int64_t b = b0 + syrk_col(tid, q);
+        const double x = shift ? v[q] - ba * c.colsum[q] - ca * c.shift[q] - nk * ba * c.shift[q] : v[q];
+        if (b < d && b >= a) G[a * d + b] = g[q] + x;
+    }
 }
 
 __global__ void __launch_bounds__(256, 1) k_syrk_f32(const float *__restrict__ T, int64_t d, int64_t d_pad,
@@ -590,12 +629,12 @@ __global__ void __launch_bounds__(256, 1) k_syrk_f32(const float *__restrict__ T
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         if (g1 - g0 == groups) {
             const double nk = (double)*n_kept;
+            SyrkCols cols;
+            syrk_cols(cols, (int64_t)bj * kBM, tid, d, shift, colsum_c);
 #pragma unroll
             for (int p = 0; p < 8; ++p)
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    syrk_add(acc64[p][q], (int64_t)bi * kBM + syrk_row(tid, p), (int64_t)bj * kBM + syrk_col(tid, q), d,
-                             shift, colsum_c, nk, G);
+                syrk_add_row(acc64[p], cols, (int64_t)bi * kBM + syrk_row(tid, p), (int64_t)bj * kBM, tid, d, shift,
+                             colsum_c, nk, G);
         } else {  // part 0 of the CTA when its run begins here, else part 1
             double *o = parts + (2 * (int64_t)blockIdx.x + (u == u0 ? 0 : 1)) * kBM * kBM + tid;
 #pragma unroll
@@ -627,9 +666,9 @@ __global__ void __launch_bounds__(256) k_syrk_f32_parts(int64_t d, int64_t m_pad
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] += o[q * 256];
     }
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-        syrk_add(v[q], (int64_t)bi * kBM + syrk_row(tid, p), (int64_t)bj * kBM + syrk_col(tid, q), d, shift, colsum_c, nk, G);
+    SyrkCols cols;
+    syrk_cols(cols, (int64_t)bj * kBM, tid, d, shift, colsum_c);
+    syrk_add_row(v, cols, (int64_t)bi * kBM + syrk_row(tid, p), (int64_t)bj * kBM, tid, d, shift, colsum_c, nk, G);
 }
 
 size_t syrk_f32_parts_bytes() { return sizeof(double) * 2 * (size_t)device_sms() * kBM * kBM; }
@@ -660,13 +699,15 @@ int launch_syrk_fold(const GramWork &w, int64_t m, const DevScale &t, double *gr
         const int64_t tiles = nb * (nb + 1) / 2;
         prof::Scope ps("syrk_fp32", st);
         CREST_TRY(ensure_smem_attr((const void *)k_syrk_f32, (size_t)kSyrkF32Smem));
-        const int64_t ctas = std::min<int64_t>(device_sms(), tiles * (m_pad / kGroupCells));
+        const int64_t ctas = syrk_ctas(tiles, m_pad / kGroupCells, device_sms());
         k_syrk_f32<<<(unsigned)ctas, 256, kSyrkF32Smem, st>>>((const float *)w.tile, w.d, w.d_pad, m_pad, nb, tiles, shift,
                                                              w.colsum_chunk, w.n_kept, gram, w.part64);
         CREST_CUDA_TRY(cudaGetLastError());
-        k_syrk_f32_parts<<<dim3((unsigned)tiles, 8), 256, 0, st>>>(w.d, m_pad, nb, tiles, ctas, shift, w.colsum_chunk,
-                                                                  w.n_kept, gram, w.part64);
-        CREST_CUDA_TRY(cudaGetLastError());
+        if (tiles % ctas) {
+            k_syrk_f32_parts<<<dim3((unsigned)tiles, 8), 256, 0, st>>>(w.d, m_pad, nb, tiles, ctas, shift, w.colsum_chunk,
+                                                                      w.n_kept, gram, w.part64);
+            CREST_CUDA_TRY(cudaGetLastError());
+        }
     } else {
         CREST_TRY(syrk_bf16x3_fold(w, m_pad, t, gram, st));
     }

@@ -33,3 +33,11 @@ def test_gram_fp32_over_runs(n, d):
     size = size + np.add.outer(shift, shift) * np.abs(S).sum(0) + n * np.outer(shift, shift)
     assert np.abs(np.triu(gram) - ref).max() <= 4e-6 * size.max()
     np.testing.assert_allclose(colsum, S.sum(0), rtol=1e-6, atol=1e-6 * n)
+
+
+@pytest.mark.parametrize("n,d", [(64, 2000), (192, 1500), (193, 1500), (2176, 2000), (2177, 2000), (40, 2050)])
+def test_gram_fp32_of_few_cells(n, d):
+    """On both sides of the line between a CTA per tile and even runs (6 groups
+    of 32 cells at 1,500 genes, 68 at 2,000, on 148 SMs), and more tiles than
+    SMs."""
+    test_gram_fp32_over_runs(n, d)
