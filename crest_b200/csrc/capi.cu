@@ -494,7 +494,8 @@ int crest_gram_accumulate(const crest_chunk *chunk, const int32_t *sub_map, int6
     CREST_TRY(upload(x->sub_map, sub_map, n_vars, st));
     DevScale ds;
     CREST_TRY(stage_scale(x->mean, x->std_, x->bias, scale, d, ds, st));
-    CREST_TRY(upload(x->gram, gram, d * d, st));
+    CREST_TRY(x->gram.ensure(8 * (size_t)std::max<int64_t>(d * d, 1)));
+    if (d) CREST_TRY(copy_in(x->gram.ptr, gram, 8 * (size_t)(d * d), st, true));
     CREST_TRY(upload(x->colsum, colsum, d, st));
     GramWork w;
     const int64_t m_cap = std::min<int64_t>(tile_cells_default(), round_up(std::max<int64_t>(s.n, 1), 64));
@@ -507,7 +508,7 @@ int crest_gram_accumulate(const crest_chunk *chunk, const int32_t *sub_map, int6
     CREST_TRY(gram_status_check(w, st));  // the caller's gram / colsum stay untouched on error
     if (precision == CREST_GRAM_BF16X3) CREST_TRY(tc_check_error());
     if (d) {
-        CREST_TRY(copy_out(gram, x->gram.ptr, 8 * (size_t)(d * d), st));
+        CREST_TRY(copy_out(gram, x->gram.ptr, 8 * (size_t)(d * d), st, true));
         CREST_CUDA_TRY(cudaMemcpyAsync(colsum, x->colsum.ptr, 8 * d, cudaMemcpyDeviceToHost, st));
     }
     CREST_CUDA_TRY(cudaStreamSynchronize(st));

@@ -26,9 +26,9 @@ inline int require_device() {
 // go through pinned buffers by several threads, others as cudaMemcpyAsync on
 // st.  copy_in may return before the transfer, with the source free to change
 // unless it is pinned; after copy_out the host data is complete once st has
-// been synchronised.
-int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st);
-int copy_out(void *host, const void *dev, size_t bytes, cudaStream_t st);
+// been synchronised.  updated: an array that one call copies both in and out.
+int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st, bool updated = false);
+int copy_out(void *host, const void *dev, size_t bytes, cudaStream_t st, bool updated = false);
 
 // host[i] += dev[i] for n doubles, or 32-bit integers when narrow (nothing when
 // host is NULL).  Made while the device still works on dev: the plain way's

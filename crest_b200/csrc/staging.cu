@@ -42,9 +42,15 @@ constexpr size_t kPiece = 1u << 20;     // 256 kB: the driver calls cost as much
 // against 1.4 / 2.4 / 3.2, into new ones 3.5 / 6.8 / 13.6 against 2.6 / 4.3 /
 // 6.5.  Sums added to the caller's (AddOut) go through the threads whatever the
 // pages: group sums of three warm arrays of 3.2 / 5.4 / 6.4 / 10.7 MB 4.4 / 4.3 /
-// 8.5 / 7.5 ms against 2.4 / 2.6 / 2.7 / 3.0.
+// 8.5 / 7.5 ms against 2.4 / 2.6 / 2.7 / 3.0.  An array that a call copies in and
+// out again goes the same way both times (the threads leave its lines in other
+// cores' caches, which a plain copy then fetches one by one): a chunk's Gram of 5.1
+// / 8 / 13.5 MB that the caller keeps 1.0 / 1.38 / 2.13 ms (300 cells) and 2.17 /
+// 2.55 / 3.31 (8,000) plain, 0.76 to 1.10 / 0.95 / 1.25 and 2.18 to 2.44 / 2.43
+// to 2.61 / 2.84 to 3.01 staged; with one way by the threads alone slower than
+// either.
 constexpr size_t kStageIn = 16u << 20, kStageOutNew = 2u << 20, kStageOutWarm = 12u << 20,
-                 kStageAdd = 2u << 20;
+                 kStageAdd = 2u << 20, kStageUpdated = 6u << 20;
 constexpr int kStageThreads = 6;        // 4 to 12 within 5 %
 constexpr int kSlots = 2 * kStageThreads;
 
@@ -161,9 +167,9 @@ bool in_pieces(const void *host, size_t bytes, cudaError_t &err, F &&work) {
 
 }  // namespace
 
-int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st) {
+int copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st, bool updated) {
     cudaError_t err = cudaSuccess;
-    const bool done = bytes >= kStageIn && in_pieces(host, bytes, err, [&](const Share &sh) {
+    const bool done = bytes >= (updated ? kStageUpdated : kStageIn) && in_pieces(host, bytes, err, [&](const Share &sh) {
         cudaError_t e = cudaSuccess;
         for (size_t i = 0; i < sh.count() && e == cudaSuccess; ++i) {
             e = cudaEventSynchronize(sh.ev[i & 1]);  // the buffer's transfer before
@@ -206,9 +212,9 @@ bool drain(const void *host, const void *dev, size_t bytes, cudaStream_t st, cud
 }
 }  // namespace
 
-int copy_out(void *host, const void *dev, size_t bytes, cudaStream_t st) {
+int copy_out(void *host, const void *dev, size_t bytes, cudaStream_t st, bool updated) {
     cudaError_t err = cudaSuccess;
-    const bool staged = stage_out(host, bytes) &&
+    const bool staged = (updated ? bytes >= kStageUpdated : stage_out(host, bytes)) &&
                         drain(host, dev, bytes, st, err, [&](const unsigned char *p, size_t at, size_t n) {
                             memcpy(static_cast<unsigned char *>(host) + at, p, n);
                         });

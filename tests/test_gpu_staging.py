@@ -154,3 +154,25 @@ def test_copies_in_from_untouched_pages(n):
         kept = np.where(gm[idx] >= 0, val, 0.0).astype(np.float64)
         assert np.array_equal(total, np.add.reduceat(kept, indptr[:-1]))
         assert np.array_equal(gt, np.bincount(gm[idx][gm[idx] >= 0], val[gm[idx] >= 0], minlength=nv))
+
+
+@pytest.mark.parametrize("d", [886, 887, 1100])  # 6,279,968 and 6,294,152 bytes: around 6 MB
+@pytest.mark.parametrize("fresh", [False, True])
+def test_gram_in_and_out_around_its_limit(d, fresh):
+    """A Gram of whole numbers added to what the caller holds, exactly: d genes
+    of 40 cells in FP64."""
+    rng = np.random.default_rng(d)
+    dense = rng.integers(0, 4, (40, d)).astype(np.float32)
+    rows, cols = np.nonzero(dense)
+    indptr = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=40))]).astype(np.int64)
+    start = 0.0 if fresh else 5.0
+    gram = np.zeros((d, d)) if fresh else np.full((d, d), start)
+    colsum = np.full(d, 3.0)
+    _native.gram_accumulate(cols.astype(np.uint32), dense[rows, cols], np.arange(40, dtype=np.int64),
+                            np.arange(d, dtype=np.int32), 0.0, False, None, indptr, 0, np.arange(d, dtype=np.int32),
+                            gram, colsum, False, None, None, 0.0)
+    want = dense.astype(np.float64).T @ dense.astype(np.float64) + start
+    iu = np.triu_indices(d)
+    assert np.array_equal(gram[iu], want[iu])
+    assert np.all(gram[np.tril_indices(d, -1)] == start)
+    assert np.array_equal(colsum, dense.sum(0, dtype=np.float64) + 3.0)
