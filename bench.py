@@ -688,7 +688,7 @@ def fused_leg(torch, peaks):
             "backward_hbm_frac": b_bwd / (b_ms / 1e3) / 1e9 / peaks["hbm_gbs"],
             "note": "backward = per-gene entry histogram and scan, the entry pass (value and size-factor "
                     "gradients, each entry's scaled value and cell written into its gene's segment) and the "
-                    "block-per-gene W gradient; bytes are the algorithmic minimum"}
+                    "W gradient by chunks of a gene's entries; bytes are the algorithmic minimum"}
 
 
 def main():

@@ -21,8 +21,9 @@
 //    step for the weakest wanted value, bounded so the block stays well
 //    conditioned for Cholesky QR;
 //  * orthonormalisation is shifted Cholesky QR (Fukaya et al. 2020) built
-//    from split-K FP64 GEMMs (k_gemm, this file; no library GEMM), Rayleigh-
-//    Ritz uses the same Jacobi kernel on the p x p projected matrix.
+//    from split-K FP64 GEMMs (this file; no library GEMM), Rayleigh-Ritz is a
+//    cyclic Jacobi on the p x p projected matrix (k_rr, eig_block.cuh, for
+//    p <= 64, else the one-CTA kernel of d <= 160).
 // Stops when every wanted residual ||C v - theta v|| <= tol * theta_1.
 #include <math.h>
 #include <stdlib.h>
